@@ -87,13 +87,15 @@ HostPlan prepareHost(Mode mode, const ParticleIO& io, const uint8_t* mask, bool 
                              hmask.data(), skipMasked, sort, symLayout, symMinLeaves, fp64Eps);
 }
 
-bool faceOnSource(int64_t nb, const double* hb, const uint8_t* hmask, double eps) {
+bool exactOnly(int64_t na, const double* ha, int64_t nb, const double* hb, const uint8_t* hmask, double eps) {
   std::vector<const double*> src;
   for (int64_t f = 0; f < nb; ++f)
     if (!hmask[f]) src.push_back(&hb[3 * (size_t)f]);
   if (src.empty()) return false;
   const double spacing2 = 4.0 * kPi / (double)src.size(), near2 = spacing2 / 400.0;
   auto onSphere = [](const double* x) { return std::fabs(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] - 1.0) <= 1e-3; };
+  for (int64_t i = 0; i < na; ++i)
+    if (!onSphere(&ha[3 * (size_t)i])) return true;
   for (int64_t f = 0; f < nb; ++f)
     if (!onSphere(&hb[3 * (size_t)f])) return true;
   if (2.0 * eps * eps >= near2) return false;  // regularised: no pair is near-singular
@@ -132,13 +134,14 @@ HostPlan prepareHostFromHost(Mode mode, int64_t na, int64_t nb, const double* ha
     kb.resize((size_t)nb);
     for (int64_t i = 0; i < nb; ++i) kb[i] = mortonKey(&hb[3 * (size_t)i]);
   }
-  bool onSource = true;
+  bool exact = true;
   if (fp64Eps >= 0.0 && hb) {
     std::vector<uint8_t> hmask((size_t)nb, 0);
     if (hmaskIn && nb > 0) std::copy(hmaskIn, hmaskIn + nb, hmask.begin());
-    if (std::count(hmask.begin(), hmask.end(), 0) >= kFP64SplitMin) onSource = faceOnSource(nb, hb, hmask.data(), fp64Eps);
+    if (std::count(hmask.begin(), hmask.end(), 0) >= kFP64SplitMin)
+      exact = exactOnly(ha ? na : 0, ha, nb, hb, hmask.data(), fp64Eps);
   }
-  return planFromKeys(mode, na, nb, ka.data(), kb.data(), hmaskIn, skipMasked, sort, symLayout, symMinLeaves, onSource);
+  return planFromKeys(mode, na, nb, ka.data(), kb.data(), hmaskIn, skipMasked, sort, symLayout, symMinLeaves, exact);
 }
 
 // ids (ascending) into the order of key(id), equal keys by id; their keys in that order.  The keys have
@@ -172,7 +175,7 @@ static void sortByKey(std::vector<int>& ids, std::vector<uint32_t>& sorted, Key 
 
 HostPlan planFromKeys(Mode mode, int64_t na, int64_t nb, const uint32_t* ka, const uint32_t* kb,
                       const uint8_t* hmaskIn, bool skipMasked, bool sort, bool symLayout, int64_t symMinLeaves,
-                      bool faceOnSource) {
+                      bool exactOnly) {
   HostPlan H;
   H.na = na;
   H.nb = nb;
@@ -187,7 +190,7 @@ HostPlan planFromKeys(Mode mode, int64_t na, int64_t nb, const uint32_t* ka, con
   const bool sym = symLayout && sort && mode != Mode::Distinct && nleaves >= std::max<int64_t>(1, symMinLeaves);
   H.symWanted = symLayout;
   H.symMin = symMinLeaves;
-  H.faceOnSource = faceOnSource;
+  H.exactOnly = exactOnly;
   std::vector<int> ids, srcFace;
   ids.reserve((size_t)(na + nb));
   srcFace.reserve((size_t)nleaves);
@@ -338,7 +341,7 @@ void buildSolve(SolvePlan& P, Mode mode, Precision prec, const ParticleIO& io, c
     S.sp1 = M.alloc<float4>(ns);
   } else {
     S.sd = M.alloc<double4_32a>(ns);
-    P.exact = ns < kFP64SplitMin || H.faceOnSource;
+    P.exact = ns < kFP64SplitMin || H.exactOnly;
     if (!P.exact) {
       S.tq = M.alloc<float4>(3 * (size_t)nslots);
       S.sq = M.alloc<float4>(3 * (size_t)ns);
@@ -907,10 +910,10 @@ std::unique_ptr<Batch> makeSingle(lpm_bve_ctx* ctx, Mode mode, Precision prec, c
   finalizeBatch(*B, ctx->dev, s);
   if (ctx->verbose)
     std::fprintf(stderr, "[lpm_bve] plan: mode=%d prec=%d slots=%d sources=%d tiles=%d chunks=%d items=%d grid=%d "
-                 "symmetric=%d (leaf0 %d, %d + %d items)\n",
+                 "split=%d sub=%d symmetric=%d (leaf0 %d, %d + %d items)\n",
                  (int)mode, (int)prec, B->solves[0]->nslots, B->solves[0]->ns, B->solves[0]->ntiles,
-                 B->solves[0]->nchunks, B->nitems, B->grid, (int)B->sym, B->solves[0]->leaf0, B->nSymDirectItems,
-                 B->nSymItems);
+                 B->solves[0]->nchunks, B->nitems, B->grid, B->nSplitItems, B->nSubItems, (int)B->sym,
+                 B->solves[0]->leaf0, B->nSymDirectItems, B->nSymItems);
   return B;
 }
 

@@ -80,7 +80,7 @@ struct SolveDev {
   int* revBad;               // [ns]
   // FP64 solves that take pairFP64Split: FP32 splits written by the prep kernel
   // (fp64_frame.hpp), else null
-  const float4* tq;          // [3][nslots] targets: digits a (3), c high | b (3), c low | c (3), scale
+  const float4* tq;          // [3][nslots] targets: digits a (3), c high | b (3), c low | c (3), unused
   const float4* sq;          // [3][ns] sources: digits a (3), W high | b (3), W low | c (3), D high
   const float* sqd;          // [ns] D low
   // FP32C batches that fill a fraction of the GPU (pairFP32CSub): the targets in FP32, written with

@@ -294,14 +294,14 @@ struct HostPlan {
   int leaf0 = -1;                  // symmetric layout: first leaf slot (-1: plain layout)
   bool symWanted = false;
   int64_t symMin = 0;
-  bool faceOnSource = true;  // FP64 RK4 (true where no positions were read)
+  bool exactOnly = true;     // FP64 (true where no positions were read)
 };
 
-// FP64 RK4 plans: whether a face (masked or not) lies within 1/20 of the mean spacing of another
-// one that is a source (with 1 - x.y + eps^2 as small), or off the sphere.  Such targets amplify the
+// FP64 plans: whether a target or face lies off the sphere, or a face (masked or not) within 1/20 of the mean
+// spacing of another one that is a source (with 1 - x.y + eps^2 as small).  Such faces amplify the
 // rounding of every source's velocity, so the plan is evaluated in the reference's own operations.
-// A fact of the faces alone: the same with and without LPM_BVE_SKIP_MASKED_TARGETS.
-bool faceOnSource(int64_t nb, const double* hb, const uint8_t* hmask, double eps);
+// A fact of the points alone: the same with and without LPM_BVE_SKIP_MASKED_TARGETS.
+bool exactOnly(int64_t na, const double* ha, int64_t nb, const double* hb, const uint8_t* hmask, double eps);
 
 // symLayout (collocated / RK4 plans, sorted): the non-leaf target slots (vertices, masked faces)
 // first in Morton order, then every leaf in source order, so that leaf slot leaf0 + k is source
@@ -311,11 +311,11 @@ bool faceOnSource(int64_t nb, const double* hb, const uint8_t* hmask, double eps
 constexpr int64_t kDeviceKeys = 32768;  // points from which a plan's Morton keys come from the device
 HostPlan prepareHost(Mode mode, const ParticleIO& io, const uint8_t* mask, bool skipMasked, bool sort,
                      cudaStream_t s, bool symLayout = false, int64_t symMinLeaves = 0, double fp64Eps = -1.0);
-// fp64Eps: the regularisation of an FP64 plan (sets faceOnSource for RK4), -1 for FP32C.
+// fp64Eps: the regularisation of an FP64 plan (sets exactOnly), -1 for FP32C.
 // Same from the points' Morton keys (host).
 HostPlan planFromKeys(Mode mode, int64_t na, int64_t nb, const uint32_t* ka, const uint32_t* kb,
                       const uint8_t* hmask, bool skipMasked, bool sort, bool symLayout, int64_t symMinLeaves,
-                      bool faceOnSource);
+                      bool exactOnly);
 // Same from host arrays: ha (na x 3) and hb (nb x 3) row-major positions, hmask (nb bytes).
 HostPlan prepareHostFromHost(Mode mode, int64_t na, int64_t nb, const double* ha, const double* hb,
                              const uint8_t* hmask, bool skipMasked, bool sort, bool symLayout = false,

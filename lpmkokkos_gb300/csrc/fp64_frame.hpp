@@ -1,17 +1,20 @@
 // fp64_frame.hpp -- how the FP64 pair kernels (pair_fp64.cu) see a point: its defect from the unit
-// sphere, the frame of a target, and the FP32 digits of its coordinates.  Device code.
+// sphere and the FP32 digits of its coordinates.  Device code.
 #pragma once
 
 #include "engine.hpp"
 
 namespace lpm {
 
-// |q| below which a pair is evaluated in the reference's operations (q = 2 (1 - x.y + eps^2); the
-// pair's distance is below 2^-6): a source and its own target, points that fall on a source.
+// q below which, or negative, a pair is evaluated in the reference's operations (q = 2 (1 - x.y + eps^2);
+// on the sphere the pair's distance is below 2^-6): a source and its own target, points that fall on
+// a source, pairs about the cone x.y = 1 of a point outside the sphere.
 constexpr double kNearQ = 0x1p-12;
-// Sources farther than this from the unit sphere (| 1 - |y|^2 |), or not finite, are evaluated in
-// the reference's operations for every target.
-constexpr double kMaxDefect = 1.0 / 16.0;
+// Sources and targets farther than this from the unit sphere (| 1 - |x|^2 |), or not finite, are
+// evaluated in the reference's operations in all their pairs.  q = |y - x|^2 + (1 - |x|^2) + (1 - |y|^2)
+// + 2 eps^2 cancels where the points lie outside: |y - x|^2, known to 2^-48 of itself, is then at most q
+// and twice this limit, so the error is 2^-52, as that of 1 - x.y in FP64.
+constexpr double kMaxDefect = 1.0 / 32.0;
 
 // 1 - |x|^2, exact to a rounding of the result for |x| near 1: the squares and their sum keep their
 // rounding errors (fused multiply-add; Knuth's two-sum).
@@ -27,33 +30,10 @@ __device__ __forceinline__ double defectOf(double x, double y, double z) {
   return __dsub_rn(1.0, s2) - lo;
 }
 
-// A source's defect, NaN where the source is not near the sphere, which makes every q with it NaN.
-__device__ __forceinline__ double sphereDefect(double x, double y, double z, double w) {
+// A point's defect, NaN where it is not near the sphere, which makes every q with it NaN.
+__device__ __forceinline__ double sphereDefect(double x, double y, double z) {
   const double d = defectOf(x, y, z);
-  return fabs(d) <= kMaxDefect && isfinite(w) ? d : __longlong_as_double(0x7ff8000000000000ll);
-}
-
-// A target as the far pairs see it: xh = 2^-k x with |xh| <= 2^0.5 (k = 0 up to |x| = 2), and
-//   q 2^-k = |y - xh|^2 + (1 - |y|^2) + c,   c = (1 - |xh|^2) + (2^(1-k) - 2) + 2 eps^2 2^-k,
-// so that a point far off the sphere keeps its digits (x cross xh = 0: the velocity takes the same
-// sums, times 2^-k).  A target that is not finite has c = NaN: every q with it is NaN.
-struct TargetFrame {
-  double x, y, z, c;
-  double scale;  // 2^-k
-  double half;   // 2^(k-1): 1 - x.y + eps^2 = (q 2^-k) half
-};
-
-__device__ __forceinline__ void targetFrame(double x, double y, double z, double eps2, TargetFrame& f) {
-  const double r2 = x * x + y * y + z * z;
-  int k = 0;
-  if (r2 > 4.0 && r2 <= 0x1p1000) k = (ilogb(r2) + 1) / 2;
-  f.scale = scalbn(1.0, -k);
-  f.half = scalbn(0.5, k);
-  f.x = x * f.scale;
-  f.y = y * f.scale;
-  f.z = z * f.scale;
-  f.c = r2 <= 0x1p1000 ? defectOf(f.x, f.y, f.z) + (k ? scalbn(2.0, -k) - 2.0 : 0.0) + 2.0 * eps2 * f.scale
-                       : __longlong_as_double(0x7ff8000000000000ll);
+  return fabs(d) <= kMaxDefect ? d : __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // x = a + b + c: a a multiple of 2^-21, b of 2^-45, |b| <= 2^-22, c the rest rounded to FP32
