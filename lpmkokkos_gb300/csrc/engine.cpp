@@ -345,7 +345,7 @@ void buildSolve(SolvePlan& P, Mode mode, Precision prec, const ParticleIO& io, c
     if (!P.exact) {
       S.tq = M.alloc<float4>(3 * (size_t)nslots);
       S.sq = M.alloc<float4>(3 * (size_t)ns);
-      S.sqd = M.alloc<float>(ns);
+      S.sqd = M.alloc<float2>(ns);
     }
   }
   if (mode == Mode::RK4) {

@@ -82,7 +82,7 @@ struct SolveDev {
   // (fp64_frame.hpp), else null
   const float4* tq;          // [3][nslots] targets: digits a (3), c high | b (3), c low | c (3), unused
   const float4* sq;          // [3][ns] sources: digits a (3), W high | b (3), W low | c (3), D high
-  const float* sqd;          // [ns] D low
+  const float2* sqd;         // [ns] D low, exponent of W (an int's bits; W high and low are W / 2^exponent)
   // FP32C batches that fill a fraction of the GPU (pairFP32CSub): the targets in FP32, written with
   // the stage positions, and the sums per sub-block of sources
   const float4* tf;          // [2][nslots] high parts, C | low parts, 1 where it can be a tile centre
@@ -105,7 +105,7 @@ struct SolveStage {
   int leaf0;                 // symmetric layout: first leaf slot (-1: none)
   unsigned long long* rev;   // [4][ns] fixed-point reverse sums (zeroed by prep), or null
   int* revBad;               // [ns]
-  float4* tq; float4* sq; float* sqd;  // FP64 splits (SolveDev), or null
+  float4* tq; float4* sq; float2* sqd;  // FP64 splits (SolveDev), or null
   const int* self;           // [nslots] source index of the same particle, -1 if none
   // pairFP32CSub batches (SolveDev), else null
   float4* tf;

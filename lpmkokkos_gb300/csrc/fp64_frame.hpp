@@ -47,6 +47,11 @@ __device__ __forceinline__ void splitDigits(double x, float& a, float& b, float&
   c = __double2float_rn(r - bd);
 }
 
+// Exponents that sources' weights are stored with, and that of no weight.  FP32 would lose weights above 2^128,
+// and digits of those below 2^-70.
+constexpr int kMinWeightExp = -1000, kMaxWeightExp = 1022, kNoWeightExp = -4000;
+__device__ __forceinline__ double powerOf2(int e) { return __hiloint2double((1023 + e) << 20, 0); }  // |e| <= 1022
+
 // v = h + l: h a multiple of 2^-28 where |v| <= 2^-4, else v rounded to FP32.
 __device__ __forceinline__ void splitDefect(double v, float& h, float& l) {
   const double hd = fabs(v) <= 0.0625 ? rint(v * 0x1p28) * 0x1p-28 : (double)__double2float_rn(v);

@@ -251,7 +251,7 @@ size_t estimateBytes(Precision prec, const PairShape& shape, bool skip, int64_t 
   const size_t nchunks = ns > 0 ? (ns + chunk - 1) / chunk : 1;
   const size_t ncomp = (size_t)pairNumComponents(prec, true);
   size_t plan = 8 * nslots + 12 * ntiles + 8 * ns + 24 * nslots + (prec == Precision::FP32C ? 64 + 28 : 32) * ns +
-                4 * 32 * nslots + 8 * nchunks * ncomp * nslots + (split ? 48 * nslots + 52 * ns : 0);
+                4 * 32 * nslots + 8 * nchunks * ncomp * nslots + (split ? 48 * nslots + 56 * ns : 0);
   const size_t bs = (size_t)stageBlockSize();
   size_t tables = 2 * (ntiles * nchunks * sizeof(WorkItem) + (2 * nslots / bs + ns / bs + 4) * sizeof(int4) +
                        sizeof(SolveDev) + sizeof(SolveStage));

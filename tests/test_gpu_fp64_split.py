@@ -151,3 +151,28 @@ def test_near_pairs_and_what_is_not_finite(oracle, capfd, psi):
     err = np.linalg.norm((u[100:200] - want).astype(float), axis=1)
     assert (err <= bound).all()
     assert np.abs(u[204:] - ref[204:]).max() <= 1e-12 * np.abs(ref[204:]).max()
+
+
+@pytest.mark.parametrize("psi", [False, True])
+def test_weights_of_any_size(capfd, psi):
+    """Weights times a power of two give the same digits, also where FP32 does not hold them; weights 80 orders of
+    magnitude apart, zero and near the ends of FP64's range stay within the bound."""
+    src, zeta, area = _cube5()
+    rng = np.random.default_rng(8)
+    tgt = _unit(rng.normal(size=(500, 3)))
+    tgt[:50] = _unit(src[:50] + 1e-3 * rng.normal(size=(50, 3)))  # near pairs
+    x, y, a, k = _dev(tgt), _dev(src), _dev(area), torch.zeros(len(src), dtype=torch.uint8, device="cuda")
+    with bve.Context(verbose=True) as c:
+        u, p = _call(c, x, y, _dev(zeta), a, k, psi)
+        assert _split_items(capfd) > 0
+        for e in (-900, -160, -130, -100, 40, 130, 900):
+            v, q = _call(c, x, y, _dev(np.ldexp(zeta, e)), a, k, psi)
+            assert np.array_equal(v, np.ldexp(u, e)), e
+            assert not psi or np.array_equal(q, np.ldexp(p, e)), e
+        mixed = zeta * np.where(rng.uniform(size=len(src)) < 0.5, 1e-42, 1e40)
+        mixed[:2000] = 0.0
+        tail = zeta * np.exp(-((np.arccos(np.clip(src @ src[17], -1, 1)) / 0.1) ** 2))
+        for z in (mixed, tail, zeta * 1e-290):
+            v, _ = _call(c, x, y, _dev(z), a, k, psi)
+            want, _, bound = _sums(tgt, src, -z * area)
+            assert (np.linalg.norm((v - want).astype(float), axis=1) <= bound).all()
