@@ -138,7 +138,7 @@ HostPlan prepareHostFromHost(Mode mode, int64_t na, int64_t nb, const double* ha
   if (fp64Eps >= 0.0 && hb) {
     std::vector<uint8_t> hmask((size_t)nb, 0);
     if (hmaskIn && nb > 0) std::copy(hmaskIn, hmaskIn + nb, hmask.begin());
-    if (std::count(hmask.begin(), hmask.end(), 0) >= kFP64SplitMin)
+    if (std::count(hmask.begin(), hmask.end(), 0) >= fp64SplitMin(mode, fp64Eps))
       exact = exactOnly(ha ? na : 0, ha, nb, hb, hmask.data(), fp64Eps);
   }
   return planFromKeys(mode, na, nb, ka.data(), kb.data(), hmaskIn, skipMasked, sort, symLayout, symMinLeaves, exact);
@@ -341,7 +341,7 @@ void buildSolve(SolvePlan& P, Mode mode, Precision prec, const ParticleIO& io, c
     S.sp1 = M.alloc<float4>(ns);
   } else {
     S.sd = M.alloc<double4_32a>(ns);
-    P.exact = ns < kFP64SplitMin || H.exactOnly;
+    P.exact = ns < fp64SplitMin(mode, eps) || H.exactOnly;
     if (!P.exact) {
       S.tq = M.alloc<float4>(3 * (size_t)nslots);
       S.sq = M.alloc<float4>(3 * (size_t)ns);

@@ -128,14 +128,21 @@ struct PairShape {
 enum class Precision { FP64 = 0, FP32C = 1 };
 
 // FP64 pair kernels (pair_fp64.cu): pairFP64Exact (items of kFP64Tile targets) and pairFP64Split
-// (items of kSplitTile), for solves of at least kFP64SplitMin sources.  The line is where the split's error
-// is no larger than that of the reference's FP64 operations (pair_fp64.cu): relative L2 of velocity and stream
-// function 1.6e-15 and 1.8e-15 against 1.6e-14 and 1.9e-15 at 6,144 sources; the stream function of
-// 5,120 sources 3.8e-15 against 1.6e-15.
+// (items of kSplitTile), which a solve takes where its error is no larger than that of the reference's FP64
+// operations (fp64SplitMin).  Relative L2 errors against 80-bit sums, split / reference, for the Rossby-Haurwitz
+// wave with up to 12 vortices:
+//   6,144 sources, eps 0: velocity 1.6e-15 / 1.5e-14 at vertices, 1.5e-15 / 5.2e-15 at faces; stream function
+//     1.9e-15 / 2.0e-15 and 1.8e-15 / 1.7e-15, level;
+//   6,144 sources, eps 0.001..0.03: velocity 0.2..0.8 of the reference's, but the stream function 1.05..1.5
+//     times it; eps 0.1 and more: velocity 1.6..3 times it;
+//   20,480 to 98,304 sources, eps 0.001..1: both 0.15..1.0 of it.
+// (A vorticity without any structure rounds less in the reference: its stream function is then off by 1.2e-15
+// against 0.5e-15 at 6,144 sources and eps 0; with eps of 0.03 and more 0.6..2e-15 against 0.2..1e-15.)
 constexpr int kFP64Threads = 256, kFP64Tile = 32, kFP64MinPerSM = 4;
 constexpr int kSplitThreads = 128, kSplitK = 2, kSplitMinB = 4;
 constexpr int kSplitTile = kSplitThreads * kSplitK;
-constexpr int kFP64SplitMin = 6144;
+constexpr int kFP64SplitMin = 6144, kFP64SplitMinEps = 20480;
+constexpr double kFP64VelocityEps = 0.03, kFP64MaxEps = 1.0;
 
 // ---- kernel launchers (pair_kernels.cu / stage_kernels.cu) ----------------------------
 // The O(N) kernels walk a block map of int4 {solve, first index, kind, 0}; kind 0 = target

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <exception>
@@ -296,6 +297,13 @@ struct HostPlan {
   int64_t symMin = 0;
   bool exactOnly = true;     // FP64 (true where no positions were read)
 };
+
+// Sources from which an FP64 solve may take pairFP64Split (engine.hpp has the errors that set the lines); RK4
+// plans sum velocities alone.
+inline int fp64SplitMin(Mode mode, double eps) {
+  if (eps == 0.0 || (mode == Mode::RK4 && std::fabs(eps) <= kFP64VelocityEps)) return kFP64SplitMin;
+  return std::fabs(eps) <= kFP64MaxEps ? kFP64SplitMinEps : INT_MAX;
+}
 
 // FP64 plans: whether a target or face lies off the sphere, or a face (masked or not) within 1/20 of the mean
 // spacing of another one that is a source (with 1 - x.y + eps^2 as small).  Such faces amplify the

@@ -176,3 +176,30 @@ def test_weights_of_any_size(capfd, psi):
             v, _ = _call(c, x, y, _dev(z), a, k, psi)
             want, _, bound = _sums(tgt, src, -z * area)
             assert (np.linalg.norm((v - want).astype(float), axis=1) <= bound).all()
+
+
+@pytest.mark.parametrize("seed,level,eps,velocity,rk4", [
+    (P.SEED_CUBED, 4, 0.0, False, False),      # 1,536 sources
+    (P.SEED_CUBED, 5, 0.0, True, True),        # 6,144
+    (P.SEED_CUBED, 5, 1e-6, False, True),
+    (P.SEED_CUBED, 5, 0.03, False, True),
+    (P.SEED_CUBED, 5, 0.031, False, False),
+    (P.SEED_ICOS_TRI, 5, 0.0, False, False),   # 20,480, parents on their children
+    (P.SEED_ICOS_TRI, 5, 0.01, True, True),
+    (P.SEED_ICOS_TRI, 5, 1.0, True, True),
+    (P.SEED_ICOS_TRI, 5, 1.01, False, False),
+    (P.SEED_ICOS_TRI, 5, 1e30, False, False),
+])
+def test_which_solves_take_the_split(oracle, capfd, seed, level, eps, velocity, rk4):
+    """The sizes and regularisations at which its error is no larger than the reference's (csrc/engine.hpp)."""
+    s = bve.BVESphere(seed, level)
+    with bve.Context(verbose=True) as c:
+        s.init_vorticity(bve.rh54_gaussians(3, 2), c, flags=P.FP64, eps=eps)
+        torch.cuda.synchronize()
+        assert (_split_items(capfd) > 0) == velocity
+        c.rk4_step(s.state(), 0.0, 0.0, 1, flags=P.FP64, eps=eps)
+        torch.cuda.synchronize()
+        assert (_split_items(capfd) > 0) == rk4
+    m = s.mesh
+    ref = oracle.velocity_distinct(m["vx"][:40], m["fx"], s.relVortFaces.cpu().numpy(), m["farea"], m["fmask"], eps=eps)
+    assert np.abs(s.velocityVerts[:40].cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
