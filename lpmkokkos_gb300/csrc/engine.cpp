@@ -391,18 +391,22 @@ void buildSolve(SolvePlan& P, Mode mode, Precision prec, const ParticleIO& io, c
 constexpr int kChunksPerTile = 8;
 constexpr int kMinChunkTiles = 4;
 
-// pairFP64Split: about 2,400 items of a solve whose targets are its own vertices and faces (1.83 per
-// source), of at least 128 sources, so that the smaller solves spread over all SMs; 8 chunks from
-// 42,000 sources on.  (Sets of over a million targets have items enough: there the chunks stay
-// few, which bounds the partial sums' memory.)
-constexpr int kSplitManySlots = 1 << 20;
+// pairFP64Split: up to 3,000 items, of at least 128 sources, so that the smaller solves spread over all SMs; 8
+// chunks from 42,000 sources or 96,000 targets on.  (64,801 points x 6,144 sources 1.37 ms, with the 48 chunks
+// that the sources alone would allow 1.37 ms; a million points 19.6 and 20.2 ms, the plan 0.34 and 1.6 GB; 200,000
+// points with the stream function 5.75 and 5.67 ms.)
+constexpr int kSplitItems = 3000;
 
 int chunkLength(const PairShape& shape, int nslots, int ns, bool split) {
   const int srcTile = shape.srcTile;
   if (ns <= 0) return srcTile;
   const int minLen = kMinChunkTiles * srcTile;
   int nch = std::max(1, std::min(kChunksPerTile, (ns + minLen - 1) / minLen));
-  if (split && nslots <= kSplitManySlots) nch = std::min(ns / 128, std::max(kChunksPerTile, 340000 / ns));
+  if (split) {
+    const int tiles = (nslots + kSplitTile - 1) / kSplitTile;
+    const int spread = std::min(340000 / ns, (kSplitItems + tiles - 1) / std::max(1, tiles));
+    nch = std::min(ns / 128, std::max(kChunksPerTile, spread));
+  }
   const int len = (ns + nch - 1) / nch;
   return (len + srcTile - 1) / srcTile * srcTile;
 }

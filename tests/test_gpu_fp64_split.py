@@ -203,3 +203,18 @@ def test_which_solves_take_the_split(oracle, capfd, seed, level, eps, velocity, 
     m = s.mesh
     ref = oracle.velocity_distinct(m["vx"][:40], m["fx"], s.relVortFaces.cpu().numpy(), m["farea"], m["fmask"], eps=eps)
     assert np.abs(s.velocityVerts[:40].cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nt,chunks", [(1, 48), (6146, 48), (16000, 48), (96000, 8), (400000, 8)])
+def test_partial_sums_stay_few_with_many_targets(capfd, nt, chunks):
+    """Small solves spread their sources over 48 chunks; sets of many targets have items enough and keep the 8
+    chunks of the other kernels, whose partial sums bound the workspace (32 bytes per target and chunk)."""
+    src, zeta, area = _cube5()
+    x = _unit(np.random.default_rng(6).normal(size=(nt, 3)))
+    mask = torch.zeros(len(src), dtype=torch.uint8, device="cuda")
+    with bve.Context(verbose=True) as c:
+        u, _ = _call(c, _dev(x), _dev(src), _dev(zeta), _dev(area), mask, False)
+        line = capfd.readouterr().err
+        v, _ = _call(c, _dev(x[:1000]), _dev(src), _dev(zeta), _dev(area), mask, False)
+    assert int(re.findall(r"split=(\d+)", line)[0]) > 0 and int(re.findall(r"chunks=(\d+)", line)[0]) == chunks
+    assert np.abs(u[:1000] - v).max() <= 1e-12 * np.abs(v).max()
