@@ -2,6 +2,8 @@
 (pairFP32CSub: targets in items of 256, sources in sub-blocks of 64, 128 x 2 or 64 x 4 threads and targets)
 against the same solve beside a large one (pairFP32C), a request alone in the server against several at
 once, and a plan sorted by keys from the device (32,768 points and more) against one sorted by the host's."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -103,3 +105,22 @@ def test_stream_function_on_a_plan_made_without_it(ctx):
         ctx.invalidate()
     assert all(np.array_equal(o[0], out[0][0]) for o in out)
     assert np.array_equal(out[1][1], out[2][1])
+
+
+@pytest.mark.parametrize("ns", [1, 63, 64, 65, 1000])
+@pytest.mark.parametrize("flags,psi", [(0, False), (0, True), (P.RCP_APPROX, False)])
+def test_sub_blocks_have_the_bits_of_the_plain_kernel(native, capfd, ns, flags, psi):
+    """Few targets against a million, whose plan takes the plain kernel: the plan lines say so."""
+    rng = np.random.default_rng(ns)
+    src, zeta, area = _points(ns, rng), rng.normal(size=ns), np.full(ns, 4 * np.pi / ns)
+    mask = np.zeros(ns, np.uint8)
+    many = _points(1 << 20, rng)
+    subs = lambda: int(re.findall(r"sub=(\d+)", capfd.readouterr().err)[-1])  # noqa: E731
+    with bve.Context(verbose=True) as c:
+        u, p = _velocity(c, many, src, zeta, area, mask, flags, psi)
+        assert subs() == 0
+        for nt in (1, 31, 255, 256, 257, 700, 200000):
+            su, sp = _velocity(c, many[:nt], src, zeta, area, mask, flags, psi)
+            assert subs() > 0
+            assert np.array_equal(su, u[:nt])
+            assert sp is None or np.array_equal(sp, p[:nt])
