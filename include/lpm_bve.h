@@ -46,7 +46,9 @@ typedef struct CUstream_st* lpm_stream_t; /* identical to cudaStream_t; NULL = l
 #define LPM_ERR_INTERNAL         (-8) /* an unexpected host-side failure (message in last_error) */
 
 /* ---- flags ------------------------------------------------------------------ */
-#define LPM_BVE_FP64                0u        /* plain FP64 pair arithmetic (the GPU oracle) */
+#define LPM_BVE_FP64                0u        /* FP64 pair arithmetic (the GPU oracle): the reference's operations, or
+                                                 where its error is no larger (from 6,144 sources on the sphere on)
+                                                 FP32 operations on exact splits */
 #define LPM_BVE_FP32C               (1u << 0) /* FP32 pair arithmetic, compensated sums, FP64 epilogue */
 #define LPM_BVE_COLLOCATED          (1u << 1) /* velocity(): targets are the sources, i == j excluded */
 #define LPM_BVE_PSI                 (1u << 2) /* also compute the stream function */
@@ -56,7 +58,8 @@ typedef struct CUstream_st* lpm_stream_t; /* identical to cudaStream_t; NULL = l
 #define LPM_BVE_RENORM              (1u << 5) /* rk4: project positions to |x| = 1 after each step */
 #define LPM_BVE_SKIP_MASKED_TARGETS (1u << 6) /* rk4: no velocity at masked faces (their x, zeta stay fixed) */
 #define LPM_BVE_NO_GRAPH            (1u << 7) /* rk4: launch kernels directly, no captured CUDA graph */
-#define LPM_BVE_NO_SORT             (1u << 8) /* keep the caller's target order (no spatial sort) */
+#define LPM_BVE_NO_SORT             (1u << 8) /* keep the caller's target order (no spatial sort); FP64: always
+                                                 the reference's operations */
 #define LPM_BVE_MESH_TARGETS        (1u << 9) /* velocity(), distinct targets: they are mesh points (e.g. the
                                                  vertices of the source mesh), each at least about half a mesh
                                                  spacing from every source.  Lets FP32C use its 13-op pair

@@ -475,9 +475,9 @@ void finalizeBatch(Batch& B, const DeviceInfo& dev, cudaStream_t s) {
   B.nitems = (int)items.size();
   B.nSplitItems = (int)split.size();
   B.slots = slots;
-  // pairFP32CSub where the plain kernel's items leave CTA slots empty (up to 0.9 of them: a single solve up to
-  // icosahedral level 4, cubed-sphere level 5, 84 items for 304 slots), or just spill into a second
-  // round (up to 1.2), as long as its sums stay below B.subLimit.  12,000 points x 20,480 sources (96
+  // pairFP32CSub where the plain kernel's items leave CTA slots empty (up to 0.9 of them filled: a single solve up
+  // to icosahedral level 4, cubed-sphere level 5, 84 items for 304 slots, some ten thousand points), or just spill
+  // into a second round (up to 1.2), as long as its sums stay below B.subLimit.  12,000 points x 20,480 sources (96
   // items): 181 us against 279; 64,801 x 5,120 (320): 250 against 294; but 64,801 x 6,144 (384) 297
   // against 294, 37,542 x 20,480 (296) 397 against 371.  The bits are the plain kernel's, so the choice is
   // free; a call for the stream function on a plan laid out without it takes the plain kernel.

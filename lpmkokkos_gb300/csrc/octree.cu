@@ -39,7 +39,7 @@ constexpr int kLevels = kOctreeMaxDepth + 1;
 constexpr double kZeroTol = 1.0e-14;  // ZERO_TOL, src/LpmDefs.hpp:99
 
 // Doubles as integers of the same order (-0 as 0): comparisons without the FP64 pipe, which takes
-// 16 times as long for one.  NaN, which no comparison holds for, is the smallest.
+// 64 times as long for one as the FP32 pipe.  NaN, which no comparison holds for, is the smallest.
 __device__ __forceinline__ long long orderOf(double v) {
   const long long b = __double_as_longlong(v);
   const long long mag = b & 0x7fffffffffffffffll;

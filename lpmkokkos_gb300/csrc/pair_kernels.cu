@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(NTH, MINB) pairFP32C(const SolveDev* __restric
   }
 }
 
-// Batches that fill a fraction of the GPU (a single solve up to icosahedral level 4): one CTA per
+// Batches that fill a fraction of the GPU (a single solve up to icosahedral level 4 or cubed-sphere level 5, or,
+// with few sources, 12,000 to 65,000 points: finalizeBatch has the line): one CTA per
 // item of kSubTile targets of a tile x one sub-block of kSub sources.  pairFP32C gives such a solve
 // one CTA per 1,024 targets and 1,024 sources or more, which leaves most SMs idle; its compensated
 // sum over a chunk's sub-blocks is a serial chain, but the sub-blocks' own FP32 sums are not.  They

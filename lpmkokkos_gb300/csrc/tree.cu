@@ -106,7 +106,7 @@ constexpr int kGeomTilesPerBlock = kBlock / 32;
 constexpr int kGeomPerLane = kTreeShape.threads * kTreeShape.k / 32;
 
 // Whether a slot's position shapes its tile: near the sphere (sane), decided in FP32 except close to
-// the bounds, where FP64 decides (an FP64 instruction takes the time of 16 FP32 ones).
+// the bounds, where FP64 decides (an FP64 instruction takes the time of 64 FP32 ones).
 __device__ __forceinline__ bool saneFast(double x, double y, double z) {
   const float fx = (float)x, fy = (float)y, fz = (float)z;
   const float r2 = fx * fx + fy * fy + fz * fz;
